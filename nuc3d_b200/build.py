@@ -86,8 +86,9 @@ def build(verbose: bool = False, force: bool = False, defines=(), out: Path | No
                "-ldl", "-lpthread"]
         subprocess.run(cmd, check=True)
     probe_src = CSRC / "probe.cu"
-    if out is None and (force or _stale(PROBE_LIB, [probe_src, Path(__file__)])):
-        subprocess.run([cc, *ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
+    if out is None and (force or _stale(PROBE_LIB, [probe_src, *headers, Path(__file__)])):
+        # (-fmad=false: the sum of ordered_sum.cuh as the reference-order build has it)
+        subprocess.run([cc, *ARCH, "-O3", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC", "-shared",
                         str(probe_src), "-o", str(PROBE_LIB), "-lcudart_static", "-lrt", "-ldl",
                         "-lpthread"], check=True)
     return LIB

@@ -17,10 +17,17 @@
 //   * evaluates each chunk's function for the predicted binade, and the segment's;
 //   * the last CTA of a block walks the segments from S = 0: where S is in the predicted
 //     binade before and after a function, S / u moves by its increment; where not (S = 0, S
-//     crosses into the next binade, a value too large, Inf or NaN) it goes down to the
-//     segment's chunks and there adds value after value.
+//     crosses into the next binade, a value too large) it goes down to the segment's chunks
+//     and there adds value after value.
 // The prediction only decides which runs take the short way: the walk checks each one, so the
 // result does not depend on it.  A look-back that gives up (kOsSpins) predicts nothing.
+// Sums that are not finite have no functions and need none: a NaN among the values makes the
+// sum NaN wherever it stands, so the CTA that meets one says so in the block's count and there
+// is no walk; and without a NaN, a sum that reaches Inf stays Inf, so the walk ends there.
+// (Walked value by value, a block that is NaN throughout took twice the plain loop's time:
+// 64^3 19.0 ms where a finite one takes 0.07.  Finite sums that the walk has to add value by
+// value over long stretches still do: S below 2^-1022, or so close below a power of two that
+// only the approximate sum passes it.)
 // One launch, each value read once.  Measured: 24^3 0.51 -> 0.07 ms, 64^3 9.0 -> 0.11 ms,
 // 128^3 78 -> 0.45 ms.  What is left is the walk: 1.5-3 us for each binade S grows through (a
 // chunk's 128 dependent additions and the loads before them; chunks of 256 and one function
@@ -37,6 +44,8 @@ constexpr int kOsSpins = 1 << 20;
 constexpr int kOsNone = 0x7fffffff;        // no function: add the values one by one
 constexpr int kOsAny = 0x7ffffffe;         // the identity in every binade (all values zero)
 constexpr unsigned long long kOsTop = 1ull << 53;
+constexpr unsigned long long kOsInf = 0x7ffull << 52;       // bits of +Inf
+constexpr unsigned kOsNanBit = 1u << 31;   // in a block's done count: a NaN among its values
 
 // The increment of S / u over a run of values for S / u even (a) and odd (b); e: the binade.
 struct Incr {
@@ -191,8 +200,8 @@ __device__ __forceinline__ OrdWork ord_work(unsigned char *w, int nblocks, int n
 __global__ void __launch_bounds__(kOsThreads)
 residual_ordered_kernel(const BlockDev *__restrict__ blocks, TileMap tm, unsigned char *work,
                         double *__restrict__ res_last, StepState *S) {
-  __shared__ int s_ticket, s_last;
-  __shared__ double s_sum[kOsChunks], s_before;
+  __shared__ int s_ticket, s_last, s_nan;
+  __shared__ double s_sum[kOsChunks];
   __shared__ Incr s_f[kOsThreads], s_g[kOsThreads / 32];
   __shared__ double s_x[kOsChunk];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -240,7 +249,10 @@ residual_ordered_kernel(const BlockDev *__restrict__ blocks, TileMap tm, unsigne
       if (lane == 0) look_put(W.look + seg, all, 1u);
       before = look_back(W.look, first, seg);
     }
-    if (lane == 0) look_put(W.look + seg, before + all, 2u);
+    if (lane == 0) {
+      look_put(W.look + seg, before + all, 2u);
+      if (all != all) atomicOr(W.done + b, kOsNanBit);  // (no term is negative: Inf alone gives no NaN)
+    }
     s_sum[lane] = before + (incl - own);
   }
   __syncthreads();
@@ -258,15 +270,17 @@ residual_ordered_kernel(const BlockDev *__restrict__ blocks, TileMap tm, unsigne
     __threadfence();
     __syncwarp();
     if (lane == 0) {
-      s_last = atomicAdd(W.done + b, 1u) == (unsigned)(end - first - 1);
+      const unsigned c = atomicAdd(W.done + b, 1u);
+      s_last = (c & ~kOsNanBit) == (unsigned)(end - first - 1);
+      s_nan = (c & kOsNanBit) != 0;
       __threadfence();
     }
   }
   __syncthreads();
   if (!s_last) return;
 
-  // the block's last CTA: from S = 0 over all its segments
-  unsigned long long s = 0;
+  // the block's last CTA: from S = 0 over all its segments, as long as S is finite
+  unsigned long long s = s_nan ? 0x7ff8ull << 48 : 0;
   for (int p = first; p < end; p += kOsThreads) {
     const int i = p + tid;
     Incr f{0, 0, kOsAny};
@@ -282,10 +296,10 @@ residual_ordered_kernel(const BlockDev *__restrict__ blocks, TileMap tm, unsigne
     if (lane == 0) s_g[warp] = f;
     __syncthreads();
     if (warp == 0) {
-      for (int g = 0; g < kOsThreads / 32; ++g) {
+      for (int g = 0; g < kOsThreads / 32 && s < kOsInf; ++g) {
         if (incr_apply(s_g[g], s)) continue;
         // segments p + 32 g + c (those past the block's last are identities)
-        for (int c = 0; c < 32; ++c) {
+        for (int c = 0; c < 32 && s < kOsInf; ++c) {
           if ((c = incr_run(s_f[32 * g + lane], c, s)) == 32) break;
           const int k = p + 32 * g + c;
           const volatile Incr *v = W.chunk + (size_t)k * kOsChunks + lane;
@@ -293,7 +307,7 @@ residual_ordered_kernel(const BlockDev *__restrict__ blocks, TileMap tm, unsigne
           h.a = v->a;
           h.b = v->b;
           h.e = v->e;
-          for (int m = 0; m < kOsChunks; ++m) {
+          for (int m = 0; m < kOsChunks && s < kOsInf; ++m) {
             if ((m = incr_run(h, m, s)) == kOsChunks) break;
             const long long at = (long long)(k - first) * kOsSeg + (long long)m * kOsChunk;
 #pragma unroll

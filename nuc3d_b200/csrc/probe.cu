@@ -8,11 +8,24 @@
 //     the same operands, for the accuracy test of the former.
 //   nuc3d_probe_crpow        the energy reset's double-double pow (cr_pow), for the test
 //     that pins its bits to the oracle's.
+//   nuc3d_probe_ordered_sum  the reference-order residual's sum of squares of given values,
+//     and its time.
 #include <cuda_runtime.h>
 
 #define NUC3D_NS fast
 #define NUC3D_FAST 1
 #include "physics.cuh"
+
+// The ordered sum on one block of given values; the sum itself takes the place of the residual.
+namespace nuc3d {
+namespace probe {
+__device__ __forceinline__ int find_block(const TileMap &, int) { return 0; }
+__device__ __forceinline__ void residual_finish(const BlockDev &, int b, double sum, double *out, StepState *) {
+  out[b] = sum;
+}
+#include "ordered_sum.cuh"
+}  // namespace probe
+}  // namespace nuc3d
 
 namespace {
 
@@ -82,6 +95,51 @@ int nuc3d_probe_qdiv(int device, const double *a, const double *b, double *q_fas
   cudaMemcpy(q_fast, d + 2 * n, bytes, cudaMemcpyDeviceToHost);
   e = cudaMemcpy(q_ieee, d + 3 * n, bytes, cudaMemcpyDeviceToHost);
   cudaFree(d);
+  return (int)e;
+}
+
+// sum[r] = v[0]^2 + v[1]^2 + ... added left to right (n a multiple of 5, host array), by launch
+// r of three on one workspace; ms: the last one's time.  Returns 0 or a CUDA error code.
+int nuc3d_probe_ordered_sum(int device, const double *v, long long n, double *sum, double *ms) {
+  using namespace nuc3d;
+  using namespace nuc3d::probe;
+  cudaError_t e = cudaSetDevice(device);
+  if (e != cudaSuccess) return (int)e;
+  if (n < 5 || n % 5) return (int)cudaErrorInvalidValue;
+  const int segs = (int)((n + kOsSeg - 1) / kOsSeg);
+  const size_t bytes = 16 + (size_t)segs * (sizeof(unsigned long long) + (1 + kOsChunks) * sizeof(Incr));
+  double *d = nullptr;
+  unsigned char *work = nullptr;
+  BlockDev *blk = nullptr;
+  if ((e = cudaMalloc(&d, (n + 1) * sizeof(double))) == cudaSuccess &&
+      (e = cudaMalloc(&work, bytes)) == cudaSuccess && (e = cudaMalloc(&blk, sizeof(BlockDev))) == cudaSuccess) {
+    BlockDev B{};
+    B.N = n / 5;
+    B.dres = d;
+    TileMap tm{};
+    tm.nblocks = 1;
+    tm.tile_start[1] = segs;
+    cudaMemcpy(d, v, n * sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemcpy(blk, &B, sizeof(B), cudaMemcpyHostToDevice);
+    cudaMemset(work, 0, bytes);
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    for (int r = 0; r < 3; ++r) {
+      cudaEventRecord(e0);
+      residual_ordered_kernel<<<segs, kOsThreads>>>(blk, tm, work, d + n, nullptr);
+      cudaEventRecord(e1);
+      e = cudaMemcpy(sum + r, d + n, sizeof(double), cudaMemcpyDeviceToHost);
+    }
+    float t = 0.0f;
+    cudaEventElapsedTime(&t, e0, e1);
+    *ms = t;
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+  }
+  cudaFree(d);
+  cudaFree(work);
+  cudaFree(blk);
   return (int)e;
 }
 
