@@ -213,13 +213,18 @@ __host__ __device__ inline long long prim_at(const int n[3], int i, int j, int k
 
 // Tiles of the gradient kernel: grad_w(nx) x grad_h(nx) cells of a z-plane (256 threads, the
 // width dividing nx evenly into at most 32: 32 x 8 for nx = 64, 24 x 10 for 24 or 48), marching
-// over a context's grad_planes z-planes.
+// over a context's grad_planes z-planes.  With its halo of 3 a tile holds at most kGradTile
+// cells, which keeps the narrowest one (nx = 4) to 48 rows.
 constexpr int kGradThreads = 256;
-__host__ __device__ inline int grad_w(int nx) {
+constexpr int kGradTile = 544;
+__host__ __device__ constexpr int grad_w(int nx) {
   const int t = (nx + 31) / 32;
   return ((nx + t - 1) / t + 3) & ~3;
 }
-__host__ __device__ inline int grad_h(int nx) { return kGradThreads / grad_w(nx); }
+__host__ __device__ constexpr int grad_h(int nx) {
+  const int w = grad_w(nx), h = kGradThreads / w, fit = kGradTile / (w + 6) - 6;
+  return h < fit ? h : fit;
+}
 __host__ __device__ inline int grad_tiles(const int n[3], int planes) {
   const int w = grad_w(n[0]), h = grad_h(n[0]);
   return ((n[0] + w - 1) / w) * ((n[1] + h - 1) / h) * ((n[2] + planes - 1) / planes);

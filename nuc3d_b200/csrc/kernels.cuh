@@ -1729,8 +1729,14 @@ __device__ __forceinline__ void visc_flux_cell(const BlockDev &B, const SolverPa
 // 4 / 6).  The zeta stencils in registers instead of the ring: 186 and 621 (spills); 8 warps
 // of 255 registers or 24 of 80 slower still; prefetch instructions and the metrics loaded
 // before the barrier: no change.
+constexpr bool grad_tiles_fit() {
+  for (int nx = 1; nx <= 512; ++nx)
+    if (grad_h(nx) < 1 || (grad_w(nx) + 6) * (grad_h(nx) + 6) > kGradTile) return false;
+  return true;
+}
+static_assert(grad_tiles_fit(), "every gradient tile fits its planes in shared memory");
 struct GradSmem {
-  static constexpr int TILE = 544;  // (W + 6) (H + 6) at most
+  static constexpr int TILE = kGradTile;  // (W + 6) (H + 6) at most
   double tile[2][4][TILE];
   double ring[8][4][kGradThreads];
 };

@@ -1,0 +1,85 @@
+"""The Navier-Stokes passes (prim_kernel, grad_kernel) against the C restatement on blocks at the
+edges of the gradient kernel's tiles: the right-hand side of the reference-order build, bit for
+bit, and of the throughput build to 1e-11 of its largest value.
+
+  * the narrowest block that is accepted (nx = 4) with more rows than one tile takes;
+  * blocks long enough along zeta for a CTA to march over 2, 4 or 8 planes, the last march
+    shorter, with tiles that nx and ny do not fill, physical zeta faces and neighbour blocks.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+PARAMS = {"Reynolds": 200.0, "Mach": 0.8, "Pt": 0.72, "Gamma": 1.4, "T_ref": 110.4, "T_inf": 288.0, "T_wall": 1.0}
+IDS = {"outlet": 1, "wall": 2, "symmetry": 3}
+PER = (None,) * 6
+
+
+def _case(shape, blocks, axis):
+    """The blocks of a perturbed vortex, cut along one axis: their states and metrics."""
+    from nuc3d_b200 import cases as C
+    whole = list(shape)
+    whole[axis] *= blocks
+    q, m = C.taylor_green(tuple(whole), mach=PARAMS["Mach"])
+    q = q * (1.0 + 0.02 * np.random.default_rng(3).uniform(-1.0, 1.0, q.shape))
+    out = []
+    for b in range(blocks):
+        at = [slice(None)] * 3
+        at[2 - axis] = slice(b * shape[axis], (b + 1) * shape[axis])
+        at = (Ellipsis,) + tuple(at)
+        out.append((np.ascontiguousarray(q[at]), {k: np.ascontiguousarray(m[k][at]) for k in
+                                                  ("jac", "xi_xyz", "eta_xyz", "zeta_xyz", "dxyz")}))
+    return out
+
+
+def _faces(b, faces, blocks, axis):
+    from nuc3d_b200 import cases as C
+    t, i = C.periodic_faces(b)
+    for f, kind in enumerate(faces):
+        if kind:
+            t[f], i[f] = -1, IDS[kind]
+    if blocks > 1:
+        t[2 * axis], t[2 * axis + 1] = (b - 1) % blocks, (b + 1) % blocks
+    return t, i
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,scheme,vis,faces,blocks,axis", [
+    ((4, 64, 8), "upwind1st", "cd2", PER, 1, 0),
+    ((4, 110, 9), "upwind1st", "cd2", ("outlet", "wall", "symmetry", "wall", None, None), 1, 0),
+    ((4, 48, 8), "upwind1st", "cd2", PER, 2, 0),
+    ((5, 53, 7), "upwind1st", "cd2", PER, 1, 0),
+    ((33, 13, 447), "weno5js", "cd6", (None,) * 4 + ("wall", "outlet"), 1, 2),   # 2 planes a march
+    ((33, 13, 447), "weno5js", "cd6", PER, 2, 2),                                # 4 planes
+    ((33, 13, 1783), "weno5js", "cd6", ("wall", "outlet", "outlet", "wall", None, None), 1, 2),  # 8 planes
+    ((33, 13, 447), "weno5js", "cd2", (None,) * 4 + ("wall", "outlet"), 1, 2),
+    ((33, 13, 447), "weno7js", "cd8", (None,) * 4 + ("wall", "outlet"), 1, 2),
+])
+def test_rhs_equals_restatement(shape, scheme, vis, faces, blocks, axis):
+    import nuc3d_b200 as nb
+    data = _case(shape, blocks, axis)
+    ref = O.Run((scheme,) * 3, "LF", "NavierStokes3d", PARAMS, vis=(vis,) * 3)
+    for b, (q, m) in enumerate(data):
+        ref.add_block(m, *_faces(b, faces, blocks, axis), None, q)
+    dt_ref, want = ref.rhs()
+    for exact in (True, False):
+        s = nb.Solver(nb.Config(scheme_ivs=(scheme,) * 3, scheme_vis=(vis,) * 3, riemann="LF",
+                                model="NavierStokes3d", reynolds=PARAMS["Reynolds"], mach=PARAMS["Mach"],
+                                prandtl=PARAMS["Pt"], t_wall=PARAMS["T_wall"], exact=exact))
+        for b, (q, m) in enumerate(data):
+            s.add_block(*shape, *_faces(b, faces, blocks, axis))
+            s.set_metrics(b, *[m[k] for k in ("jac", "xi_xyz", "eta_xyz", "zeta_xyz", "dxyz")])
+        s.finalize()
+        for b, (q, _) in enumerate(data):
+            s.set_q(b, q)
+        dt = s.rhs()
+        for b in range(blocks):
+            got = s.get_rhs(b)
+            if exact:
+                assert dt == dt_ref
+                assert np.array_equal(got, want[b]), float(np.max(np.abs(got - want[b])))
+            else:
+                for v in range(5):
+                    assert np.max(np.abs(got[v] - want[b][v])) <= 1e-11 * np.max(np.abs(want[b])), v
+        s.close()
