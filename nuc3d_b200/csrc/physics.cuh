@@ -35,8 +35,9 @@ __device__ __forceinline__ double qdiv(double a, double b) {
 // compiler from overlapping what surrounds it): the PTX reciprocal square root r0, one coupled
 // Newton step for g ~ sqrt(x) and h ~ 1 / (2 sqrt(x)) (R. Goldschmidt, MIT thesis, 1964), and
 // the residual correction g + (x - g^2) h (P. Markstein, IBM J. Res. Dev. 34(1), 1990), within
-// an ulp.  Arguments below 2^-900 (r0 flushes subnormals) are scaled by 2^240 first; 0 gives 0,
-// Inf gives NaN.
+// an ulp.  Arguments below 2^-900 (r0 flushes subnormals) are scaled by 2^240 first; 0 and Inf
+// are their own roots (an Inf sound speed has to reach the largest eigenvalue, which a NaN
+// would not: dt becomes 0), told from the high word, off the FP64 pipe.
 __device__ __forceinline__ double qsqrt(double x) {
   const bool tiny = x < 0x1p-900;
   const double y = tiny ? x * 0x1p240 : x;
@@ -47,7 +48,8 @@ __device__ __forceinline__ double qsqrt(double x) {
   g = fma(g, e, g);
   h = fma(h, e, h);
   g = fma(fma(-g, g, y), h, g);
-  return y == 0.0 ? 0.0 : (tiny ? g * 0x1p-120 : g);
+  const int hi = __double2hiint(y);
+  return (hi << 1) == 0 || hi == 0x7ff00000 ? y : (tiny ? g * 0x1p-120 : g);
 }
 #endif
 
