@@ -120,13 +120,19 @@ compact_march_kernel(const BlockDev *__restrict__ blocks, TileMap tm, SolverPara
       const int k = min(physL ? f : R, physR ? L - f : R);  // faces to a physical one (R: none near)
       if (f <= R || f >= L - R) {
         // faces next to the ends and the system's end rows are explicit: rows 0 1 0 | h
-        cp[0] = cp[1] = 0.0;
+        double h[2];
         if (k < R) {
-          dp[0] = k == 0 ? wp[2] : (k == 1 ? rb_second(wp[2], wp[3]) : rb_third(wp[1], wp[2], wp[3]));
-          dp[1] = k == 0 ? wn[2] : (k == 1 ? rb_second(wn[2], wn[1]) : rb_third(wn[3], wn[2], wn[1]));
+          h[0] = k == 0 ? wp[2] : (k == 1 ? rb_second(wp[2], wp[3]) : rb_third(wp[1], wp[2], wp[3]));
+          h[1] = k == 0 ? wn[2] : (k == 1 ? rb_second(wn[2], wn[1]) : rb_third(wn[3], wn[2], wn[1]));
         } else {
-          dp[0] = weno5js(wp[0], wp[1], wp[2], wp[3], wp[4]);
-          dp[1] = weno5js(wn[4], wn[3], wn[2], wn[1], wn[0]);
+          h[0] = weno5js(wp[0], wp[1], wp[2], wp[3], wp[4]);
+          h[1] = weno5js(wn[4], wn[3], wn[2], wn[1], wn[0]);
+        }
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          // (the system's last row: a NaN of the rows before reaches it, as by the elimination)
+          dp[z] = f == L - R ? h[z] - 0.0 * (dp[z] + cp[z]) : h[z];
+          cp[z] = 0.0;
         }
       } else {
         const double s0[5] = {wp[0], wp[1], wp[2], wp[3], wp[4]}, s1[5] = {wn[4], wn[3], wn[2], wn[1], wn[0]};
@@ -176,8 +182,11 @@ compact_march_kernel(const BlockDev *__restrict__ blocks, TileMap tm, SolverPara
       if (rk) nu = __ldg(q + v * N + idx);
       if (un_read) nn = q0[v * N + idx];
     }
-    xp = a[1] - a[0] * xp;
-    xm = a[3] - a[2] * xm;
+    // (the faces outside the system, f < R and f > L - R, and its last row have no next face: times
+    // a zero, a NaN or Inf of that face would reach them)
+    const bool in = f >= R && f < L - R;
+    xp = in ? a[1] - a[0] * xp : a[1];
+    xm = in ? a[3] - a[2] * xm : a[3];
     const double h = xp + xm;
     if (f < L && live) {
       const long long idx = cell0 + f * sL;
