@@ -1729,6 +1729,9 @@ __device__ __forceinline__ void visc_flux_cell(const BlockDev &B, const SolverPa
 // 4 / 6).  The zeta stencils in registers instead of the ring: 186 and 621 (spills); 8 warps
 // of 255 registers or 24 of 80 slower still; prefetch instructions and the metrics loaded
 // before the barrier: no change.
+// CD6 false: cd2 and cd8 in any direction, chosen per direction at run time.  cd2 reads the same
+// planes; cd8's two outermost values come from memory (a fourth halo cell would cost the planes'
+// shared memory and the ring a ninth plane).
 constexpr bool grad_tiles_fit() {
   for (int nx = 1; nx <= 512; ++nx)
     if (grad_h(nx) < 1 || (grad_w(nx) + 6) * (grad_h(nx) + 6) > kGradTile) return false;
@@ -1742,14 +1745,14 @@ struct GradSmem {
 };
 
 // The four primitives' differences at line position c, f at the cell, near a physical face (the
-// one-sided schemes, which read no ghost) or with a scheme the fast path does not unroll.
-// Out of line, so that the common path stays small.
+// one-sided schemes, which read no ghost).  Out of line, so that the common path stays small.
 __device__ __noinline__ void grad_edge(const double *__restrict__ f, long long NP, long long s, int c, int L,
                                        int ts, bool pl, bool pr, int vis, double *out) {
   for (int v = 0; v < 4; ++v, f += NP)
     out[v] = diff_at(c, L, ts, pl, pr, vis, [f, c, s](int g) { return __ldg(f + (g - c) * s); });
 }
 
+template <bool CD6>
 __global__ void __launch_bounds__(kGradThreads, 2)
 grad_kernel(const BlockDev *__restrict__ blocks, TileMap tm, SolverParams P, int planes) {
   extern __shared__ double smem[];
@@ -1786,7 +1789,7 @@ grad_kernel(const BlockDev *__restrict__ blocks, TileMap tm, SolverParams P, int
   auto inner = [&](int d, int c) {  // not within ts cells of a physical face
     return (!phys(2 * d) || c >= P.ts[d]) && (!phys(2 * d + 1) || c < n[d] - P.ts[d]);
   };
-  const bool fast[3] = {P.vis[0] == VIS_CD6 && inner(0, i), P.vis[1] == VIS_CD6 && inner(1, j), P.vis[2] == VIS_CD6};
+  const bool fast[2] = {inner(0, i), inner(1, j)};
   // the ring holds planes k-3 .. k+3 (and k+4 on its way); k & 7 of a negative k is still 0..7
   for (int k = k0 - 3; k < k0 + 3; ++k) load_ring(k);
   load_tile(k0);
@@ -1809,29 +1812,33 @@ grad_kernel(const BlockDev *__restrict__ blocks, TileMap tm, SolverParams P, int
 #pragma unroll
         for (int v = 0; v < 4; ++v) gr[v][d] = g4[v];
       };
+      // direction d's difference of component c; V(x): the value x cells on, |x| <= 3
+      auto diff = [&](int d, int c, auto V) -> double {
+        if (!CD6 && P.vis[d] == VIS_CD2) return cd2(V(-1), V(1));
+        if (!CD6 && P.vis[d] == VIS_CD8) {
+          const long long s = d == 0 ? 1 : (d == 1 ? sy : sz);
+          const double *f = p + (k - k0) * sz + c * NP;
+          return cd8(__ldg(f - 4 * s), V(-3), V(-2), V(-1), V(1), V(2), V(3), __ldg(f + 4 * s));
+        }
+        return cd6(V(-3), V(-2), V(-1), V(1), V(2), V(3));
+      };
       const double(*T)[GradSmem::TILE] = sm.tile[k & 1];
       const int o = (r + 3) * cols + x + 3;
       if (fast[0]) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          gr[c][0] = cd6(T[c][o - 3], T[c][o - 2], T[c][o - 1], T[c][o + 1], T[c][o + 2], T[c][o + 3]);
+        for (int c = 0; c < 4; ++c) gr[c][0] = diff(0, c, [&](int a) { return T[c][o + a]; });
       } else {
         edge(0, i);
       }
       if (fast[1]) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          gr[c][1] = cd6(T[c][o - 3 * cols], T[c][o - 2 * cols], T[c][o - cols], T[c][o + cols],
-                         T[c][o + 2 * cols], T[c][o + 3 * cols]);
+        for (int c = 0; c < 4; ++c) gr[c][1] = diff(1, c, [&](int a) { return T[c][o + a * cols]; });
       } else {
         edge(1, j);
       }
-      if (fast[2] && inner(2, k)) {
+      if (inner(2, k)) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          auto V = [&](int z) { return sm.ring[(k + z) & 7][c][tid]; };
-          gr[c][2] = cd6(V(-3), V(-2), V(-1), V(1), V(2), V(3));
-        }
+        for (int c = 0; c < 4; ++c) gr[c][2] = diff(2, c, [&](int a) { return sm.ring[(k + a) & 7][c][tid]; });
       } else {
         edge(2, k);
       }
@@ -2253,8 +2260,10 @@ inline cudaError_t launch_viscous(const Launch &L, int stage) {
                                                             L.d_state, stage);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  grad_kernel<<<L.tm_grad.tile_start[L.tm_grad.nblocks], kGradThreads, sizeof(GradSmem), L.stream>>>(
-      L.d_blocks, L.tm_grad, L.P, L.grad_planes);
+  const bool cd6 = L.P.vis[0] == VIS_CD6 && L.P.vis[1] == VIS_CD6 && L.P.vis[2] == VIS_CD6;
+  (cd6 ? grad_kernel<true> : grad_kernel<false>)
+      <<<L.tm_grad.tile_start[L.tm_grad.nblocks], kGradThreads, sizeof(GradSmem), L.stream>>>(L.d_blocks, L.tm_grad,
+                                                                                              L.P, L.grad_planes);
   return cudaGetLastError();
 }
 
@@ -2547,9 +2556,11 @@ inline cudaError_t configure_dir() {
 }
 
 cudaError_t configure() {
-  cudaError_t e = cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(GradSmem));
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
+  for (auto kernel : {grad_kernel<true>, grad_kernel<false>}) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem));
+    if (e != cudaSuccess) return e;
+  }
   if ((e = configure_dir<0>()) != cudaSuccess) return e;
   if ((e = configure_dir<1>()) != cudaSuccess) return e;
   return configure_dir<2>();
