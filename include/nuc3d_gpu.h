@@ -275,12 +275,15 @@ int nuc3d_autotune(nuc3d_ctx *ctx, int reps, int shape_out[3], double ms_out[9])
    next tiles' state, Jacobian and metric with tensor-map (TMA) copies while the other warps
    compute (Navier-Stokes: the viscous fluxes by plain loads); results are identical either
    way.  Switched on, a direction may run pipelined where its blocks have an even nx (16-byte
-   rows) and an explicit scheme, and does where the kernel was measured to be no slower: the
-   throughput build's zeta sweep of the schemes other than WENO5 (whose eta and zeta sweeps
-   march along the lines from 2^18 cells on).  on = 1: every direction; on > 1: the directions
-   of its bits 0..2 (bit d: direction d); 0: none.  nuc3d_autotune also chooses, per
-   direction, between on and off.  nuc3d_get_pipeline: the directions switched on in a context
-   whose blocks allow it (bit d), 0 for none. */
+   rows) and an explicit scheme, and a launch does where the kernel was measured to be no
+   slower: upwind1st; weno3js of the throughput build (along xi in stage 0 only), and of the
+   reference-order build in small launches and Euler blocks along zeta; the throughput build's
+   zeta; and launches of a tile for every other SM at most (throughput build: eta).  The throughput build's WENO5 eta and zeta
+   sweeps of 2^18 cells or more march along the lines instead.  on = 1: every direction; on > 1:
+   the directions of its bits 0..2 (bit d: direction d); 0: none.  nuc3d_autotune also chooses,
+   per direction, between on and off.  nuc3d_get_pipeline: the directions that may run pipelined
+   in the context (bit d: switched on, even nx, a pipelined kernel, and no march over the whole
+   context), 0 for none. */
 int nuc3d_set_pipeline(nuc3d_ctx *ctx, int on);
 int nuc3d_get_pipeline(nuc3d_ctx *ctx, int *on);
 

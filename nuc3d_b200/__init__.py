@@ -380,8 +380,8 @@ class Solver:
         _check(self.lib.nuc3d_set_pipeline(self._ctx, v))
 
     def pipeline(self) -> int:
-        """Directions (bit d) whose sweeps run pipelined (even nx, explicit schemes, switched on);
-        0 for none."""
+        """Directions (bit d) whose sweeps may run pipelined (switched on, even nx, not marching;
+        a launch does where that kernel is the faster one); 0 for none."""
         v = ctypes.c_int()
         _check(self.lib.nuc3d_get_pipeline(self._ctx, ctypes.byref(v)))
         return v.value

@@ -237,6 +237,10 @@ __host__ __device__ inline int grad_tiles(const int n[3], int planes) {
 // 256^3 859 / 1212; zeta 64^3 28 / 28, 128^3 140 / 162, 256^3 915 / 1232.
 constexpr long long kMarchMin = 1ll << 18;
 
+// The kernels of an explicit direction's sweep: one tile per CTA (TILES_NOW: a launch of another
+// size may be pipelined), pipelined, marching.
+enum SweepKind : int { SWEEP_TILES = 0, SWEEP_TILES_NOW = 1, SWEEP_PIPE = 2, SWEEP_MARCH = 3 };
+
 // What the host hands to a stage launch.
 struct Launch {
   const BlockDev *d_blocks;
@@ -255,7 +259,7 @@ struct Launch {
   // memory and the persistent grid (CTAs); null / 0: the one-tile-per-CTA sweeps
   const CUtensorMap *d_maps;
   int pipe_grid;
-  int pipe_dirs;           // bit d: direction d runs pipelined (nuc3d_autotune picks per direction)
+  int pipe_dirs;           // bit d: direction d may run pipelined (nuc3d_autotune picks per direction)
   // each block's residual root of the previous step (the reference's static res_last);
   // null: no residual (nuc3d_rhs_noalloc)
   double *d_res_last;
@@ -325,6 +329,8 @@ cudaError_t run_metrics(const double *x, const double *y, const double *z, const
                         double *jac, double *met, double *dxyz, unsigned *bad, cudaStream_t st);
 cudaError_t run_diag(const Launch &L, const DiagDev *dd, double *sums, double *parts);
 cudaError_t run_sweep(const Launch &L, int dir, int stage, int flags);
+// sweep_kind(): the kernel a launch of direction dir takes (SweepKind; without the eigenvalues).
+int sweep_kind(const Launch &L, int dir);
 // run_taps(): debug taps of direction dir for one block (nl: its lines along dir);
 // out = FluxL, FluxR (5N), reconstFluxL, reconstFluxR (5 (L+1) nl), dF (5N), device.
 cudaError_t run_taps(const Launch &L, int block, int dir, int nl, double *const out[5]);
@@ -358,6 +364,8 @@ cudaError_t run_metrics(const double *x, const double *y, const double *z, const
                         double *jac, double *met, double *dxyz, unsigned *bad, cudaStream_t st);
 cudaError_t run_diag(const Launch &L, const DiagDev *dd, double *sums, double *parts);
 cudaError_t run_sweep(const Launch &L, int dir, int stage, int flags);
+// sweep_kind(): the kernel a launch of direction dir takes (SweepKind; without the eigenvalues).
+int sweep_kind(const Launch &L, int dir);
 // run_taps(): debug taps of direction dir for one block (nl: its lines along dir);
 // out = FluxL, FluxR (5N), reconstFluxL, reconstFluxR (5 (L+1) nl), dF (5N), device.
 cudaError_t run_taps(const Launch &L, int block, int dir, int nl, double *const out[5]);

@@ -2131,14 +2131,53 @@ __host__ __device__ constexpr size_t hybrid_smem_bytes(bool ns) {
          (NUC3D_HYB_PREFETCH ? rhs_stage_bytes<DIR>(ns) : 0);
 }
 
-// Directions whose sweep may run pipelined.  The one-tile-per-CTA sweep, with twice the warps
-// per SM, is the faster one along xi and eta at every size and in every direction of the
-// reference-order build (us, pipelined / tiles: throughput xi WENO5-Z 64^3 35.0 / 28.8, 256^3
-// 1207 / 957, Navier-Stokes 256^3 1436 / 1179; eta WENO7 96^3 153 / 120, 256x256x128 1013 /
-// 836; reference-order WENO5-Z 128^3 xi 561 / 392, eta 503 / 404, zeta 445 / 356, Navier-
-// Stokes 64^3 60 / 49, 56 / 50, 58 / 57).  The throughput build's zeta is close (WENO7
-// 76x52x60 42.6 / 44.8, 256x256x128 973 / 946) and stays a choice.
-template <int DIR> constexpr bool kPipeDir = NUC3D_FAST && DIR == 2;
+// Cells of a launch.
+template <int DIR> inline long long launch_cells(const Launch &L) {
+  const BlockDev *h = L.h_blocks;
+  if (L.k1 > 0) return (long long)h[0].n[0] * h[0].n[1] * (L.k1 - L.k0);
+  long long n = 0;
+  for (int b = L.b0; b < (L.b1 > 0 ? L.b1 : L.tm_dir[DIR].nblocks); ++b) n += h[b].N;
+  return n;
+}
+
+// Which launches run pipelined (pipe_sweep_kernel) where they may.  It has half the warps per SM
+// of the one-tile-per-CTA sweep, but TMA brings its tiles, so it wins
+//   * where a scheme has little arithmetic: upwind1st everywhere (right-hand side, us, pipelined /
+//     tiles: reference-order Euler 64^3 108 / 130, 128^3 471 / 676, Navier-Stokes 128^3 1052 /
+//     1231; throughput Euler 64^3 80 / 90, 128^3 277 / 421, Navier-Stokes 128^3 727 / 869);
+//     weno3js of the throughput build (Euler 128^3 361 / 464, Navier-Stokes 765 / 911), along xi
+//     only with the eigenvalues, whose metrics the tiles wait for (without: 64^3 18.6 / 16.6,
+//     128^3 99 / 107); and weno3js of the reference-order build in launches of at most a tile per
+//     resident CTA (32^3 Euler 72 / 80, Navier-Stokes 96 / 109);
+//   * where a launch has a tile for every other SM at most: its time is then one tile's latency.
+//     Steps of 16^3, one context alone and three overlapping, per step: reference-order weno5js
+//     Navier-Stokes 211 / 225 and 76 / 80, WENO5-Z Euler 167 / 177 and 60 / 63; throughput eta
+//     58 / 60 and 23.5 / 24.1.  With more tiles only the context alone gains (32^3 256 / 281), and
+//     overlapping ones lose more, their CTAs having to share the SMs (147 / 128), so the line is
+//     there.  Not the throughput build's xi (16^3 6.8 / 6.3) nor the reference-order WENO7 xi and
+//     zeta of Euler (18.2 / 16.5, 18.0 / 17.4).
+// With more tiles and more arithmetic it is the slower one (reference-order WENO5-Z 64^3 xi 66 /
+// 55, eta 63 / 54, zeta 60 / 53, 128^3 440 / 364, 414 / 353, 390 / 358; throughput WENO7 128^3 xi
+// 268 / 212, eta 249 / 213).  Close to even: the throughput build's zeta, pipelined (WENO7 64^3
+// Navier-Stokes 45 / 41, 128^3 303 / 318, 8 blocks of 40x36x44 80 / 92), and the reference-order
+// weno3js of Euler, pipelined along zeta and, with the eigenvalues, xi where the tiles are at
+// least half full (right-hand side 128^3 813 / 848, 8 blocks of 40x36x44 312 / 330; tiles a
+// quarter full, 27 blocks of 16^3: 179 / 166; Navier-Stokes 64^3 250 / 242).
+template <int DIR, int SCH>
+constexpr bool kPipe = !NUC3D_FAST || DIR != 0 || SCH == SCH_UPWIND1 || SCH == SCH_WENO3JS;
+template <int DIR, int SCH> inline bool pipe_pays(const Launch &L, int ntiles, int flags) {
+  const bool ns = (flags & SW_NS) != 0, eig = (flags & SW_EIG) != 0;
+  if (SCH == SCH_UPWIND1 || (NUC3D_FAST && DIR == 2)) return true;
+  if (NUC3D_FAST && SCH == SCH_WENO3JS) return DIR == 1 || eig;
+  if (4 * ntiles <= L.pipe_grid) return DIR == 1 || (!NUC3D_FAST && (ns || SCH != SCH_WENO7JS));
+  if (NUC3D_FAST || SCH != SCH_WENO3JS) return false;
+  if (ntiles <= L.pipe_grid) return true;
+  return !ns && (DIR == 2 || (DIR == 0 && eig)) && 2 * launch_cells<DIR>(L) >= 256ll * ntiles;
+}
+template <int DIR, int SCH> inline bool may_pipe(const Launch &L) {
+  return kPipe<DIR, SCH> && L.d_maps && L.pipe_grid > 0 && ((L.pipe_dirs >> DIR) & 1) &&
+         !(SCH == SCH_WENO5Z && L.P.sensor);
+}
 
 template <int DIR, int SCH, int SHP>
 inline cudaError_t launch_sweep_s(const Launch &L, int stage, int flags) {
@@ -2154,9 +2193,9 @@ inline cudaError_t launch_sweep_s(const Launch &L, int stage, int flags) {
     }
   }
 #endif
-  if (kPipeDir<DIR> && L.d_maps && L.pipe_grid > 0 && ((L.pipe_dirs >> DIR) & 1)) {
-    // persistent sweep fed by tensor-map loads (sweep_pipe.cuh)
-    if constexpr (kPipeDir<DIR>) {
+  if constexpr (kPipe<DIR, SCH>) {
+    if (may_pipe<DIR, SCH>(L) && pipe_pays<DIR, SCH>(L, ntiles, flags)) {
+      // persistent sweep fed by tensor-map loads (sweep_pipe.cuh)
       const int grid = ntiles < L.pipe_grid ? ntiles : L.pipe_grid;
       if (ns)
         pipe_sweep_kernel<DIR, SCH, SHP, true><<<grid, kPipeThreads, PipeSmem<DIR, SCH, SHP, true>::TOTAL,
@@ -2165,8 +2204,8 @@ inline cudaError_t launch_sweep_s(const Launch &L, int stage, int flags) {
       else
         pipe_sweep_kernel<DIR, SCH, SHP><<<grid, kPipeThreads, PipeSmem<DIR, SCH, SHP>::TOTAL, L.stream>>>(
             L.d_blocks, L.d_maps, L.tm_dir[DIR], L.P, L.d_state, stage, flags);
+      return cudaGetLastError();
     }
-    return cudaGetLastError();
   }
   const size_t smem = sweep_smem_bytes<DIR, SCH, SHP>(ns) + rhs_stage_bytes<DIR>(ns);
   sweep_kernel<DIR, SCH, false, SHP><<<ntiles, kThreads, smem, L.stream>>>(L.d_blocks, L.tm_dir[DIR], L.P,
@@ -2174,11 +2213,17 @@ inline cudaError_t launch_sweep_s(const Launch &L, int stage, int flags) {
   return cudaGetLastError();
 }
 
+#if NUC3D_FAST
+template <int DIR> inline bool runs_marching(const Launch &L) {
+  return march_dir(L.P, DIR) && (DIR == 2 ? L.march_zeta : launch_cells<DIR>(L) >= kMarchMin);
+}
+#endif
+
 template <int DIR, int SCH>
 inline cudaError_t launch_sweep_t(const Launch &L, int stage, int flags) {
 #if NUC3D_FAST
   if constexpr (DIR != 0 && (SCH == SCH_WENO5JS || SCH == SCH_WENO5Z)) {
-    if (march_dir(L.P, DIR) && (DIR == 2 ? L.march_zeta : march_cells<DIR>(L) >= kMarchMin))
+    if (runs_marching<DIR>(L))
       return (flags & SW_NS) ? launch_march<DIR, SCH, true>(L, stage, flags)
                              : launch_march<DIR, SCH, false>(L, stage, flags);
   }
@@ -2460,6 +2505,29 @@ cudaError_t run_diag(const Launch &L, const DiagDev *dd, double *sums, double *p
   return cudaGetLastError();
 }
 
+template <int DIR, int SCH> inline int sweep_kind_s(const Launch &L) {
+  if (!may_pipe<DIR, SCH>(L)) return SWEEP_TILES;
+  const int flags = L.P.model == MODEL_NS ? SW_NS : 0;
+  return pipe_pays<DIR, SCH>(L, tile_range(L.tm_dir[DIR]), flags) ? SWEEP_PIPE : SWEEP_TILES_NOW;
+}
+template <int DIR> inline int sweep_kind_d(const Launch &L) {
+#if NUC3D_FAST
+  if constexpr (DIR != 0)
+    if (runs_marching<DIR>(L)) return SWEEP_MARCH;
+#endif
+  switch (L.P.scheme[DIR]) {
+    case SCH_WENO5JS: return sweep_kind_s<DIR, SCH_WENO5JS>(L);
+    case SCH_WENO5Z: return sweep_kind_s<DIR, SCH_WENO5Z>(L);
+    case SCH_WENO7JS: return sweep_kind_s<DIR, SCH_WENO7JS>(L);
+    case SCH_WENO3JS: return sweep_kind_s<DIR, SCH_WENO3JS>(L);
+    case SCH_UPWIND1: return sweep_kind_s<DIR, SCH_UPWIND1>(L);
+    default: return SWEEP_TILES;
+  }
+}
+int sweep_kind(const Launch &L, int dir) {
+  return dir == 0 ? sweep_kind_d<0>(L) : dir == 1 ? sweep_kind_d<1>(L) : sweep_kind_d<2>(L);
+}
+
 cudaError_t run_sweep(const Launch &L, int dir, int stage, int flags) {
   const int f = flags | (L.P.model == MODEL_NS ? SW_NS : 0);
   if (L.bc_tiles > 0) {
@@ -2490,7 +2558,7 @@ inline cudaError_t configure_s() {
   static_assert(PipeSmem<DIR, SCH, SHP>::TOTAL <= kSmemOptin, "pipelined tile fits");
   static_assert(hybrid_smem_bytes<DIR, SCH, SHP>(true) <= kSmemOptin, "hybrid tile fits");
   cudaError_t e = cudaSuccess;
-  if constexpr (kPipeDir<DIR>) {
+  if constexpr (kPipe<DIR, SCH>) {
     e = cudaFuncSetAttribute(pipe_sweep_kernel<DIR, SCH, SHP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)PipeSmem<DIR, SCH, SHP>::TOTAL);

@@ -1227,6 +1227,11 @@ static int apply_shapes(nuc3d_ctx *c, const int shape[3]) {
   return build_maps(c);
 }
 
+// The kernel of direction d's sweep over the whole context.
+static int sweep_kind(const nuc3d_ctx *c, int d) {
+  return c->exact ? nuc3d::exact::sweep_kind(c->L, d) : nuc3d::fast::sweep_kind(c->L, d);
+}
+
 static bool compact_scheme(int s) { return s == SCH_CRWENO5 || s == SCH_HCCS || s == SCH_HCCS77; }
 
 int nuc3d_set_tiles(nuc3d_ctx *c, const int shape[3]) {
@@ -1617,7 +1622,9 @@ int nuc3d_get_compact_solver(nuc3d_ctx *c, int *dirs) {
 
 int nuc3d_get_pipeline(nuc3d_ctx *c, int *on) {
   if (!c || !on) return fail(NUC3D_EINVAL, "null argument");
-  *on = c->L.d_maps != nullptr ? c->L.pipe_dirs : 0;
+  *on = 0;
+  for (int d = 0; d < 3 && c->finalized; ++d)
+    if (const int k = sweep_kind(c, d); k == SWEEP_PIPE || k == SWEEP_TILES_NOW) *on |= 1 << d;
   return NUC3D_OK;
 }
 

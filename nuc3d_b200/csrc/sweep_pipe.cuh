@@ -1,6 +1,6 @@
 // sweep_pipe.cuh -- the explicit-scheme sweep as a persistent, warp-specialised kernel fed
 // by the Tensor Memory Accelerator (included by kernels.cuh inside its namespace).  It runs
-// where it is no slower than the other sweeps: kPipeDir in kernels.cuh.
+// where it is no slower than the other sweeps: pipe_pays in kernels.cuh.
 //
 // Same arithmetic as sweep_kernel (phases split -> faces -> cells, the reference's
 // operations: src/physicsModel.cpp:420-760, src/euler3d.cpp:305-366, :143-241, :368-427,
