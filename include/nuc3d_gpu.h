@@ -276,9 +276,10 @@ int nuc3d_autotune(nuc3d_ctx *ctx, int reps, int shape_out[3], double ms_out[9])
    compute (Navier-Stokes: the viscous fluxes by plain loads); results are identical either
    way.  Switched on, a direction may run pipelined where its blocks have an even nx (16-byte
    rows) and an explicit scheme, and a launch does where the kernel was measured to be no
-   slower: upwind1st; weno3js of the throughput build (along xi in stage 0 only), and of the
-   reference-order build in small launches and Euler blocks along zeta; the throughput build's
-   zeta; and launches of a tile for every other SM at most (throughput build: eta).  The throughput build's WENO5 eta and zeta
+   slower: upwind1st; weno3js of the throughput build along eta, and along stage 0's xi of large
+   launches, and of the reference-order build in launches of at most two tiles per SM; the
+   throughput build's zeta; and launches of a tile for every other SM at most (throughput build:
+   eta).  The throughput build's WENO5 eta and zeta
    sweeps of 2^18 cells or more march along the lines instead.  on = 1: every direction; on > 1:
    the directions of its bits 0..2 (bit d: direction d); 0: none.  nuc3d_autotune also chooses,
    per direction, between on and off.  nuc3d_get_pipeline: the directions that may run pipelined

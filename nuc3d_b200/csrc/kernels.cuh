@@ -1731,7 +1731,8 @@ __device__ __forceinline__ void visc_flux_cell(const BlockDev &B, const SolverPa
 // before the barrier: no change.
 // CD6 false: cd2 and cd8 in any direction, chosen per direction at run time.  cd2 reads the same
 // planes; cd8's two outermost values come from memory (a fourth halo cell would cost the planes'
-// shared memory and the ring a ninth plane).
+// shared memory and the ring a ninth plane).  128^3, reference-order and throughput, with every
+// stencil from memory / now: cd2 260 / 183 and 229 / 150, cd8 302 / 271 and 268 / 231.
 constexpr bool grad_tiles_fit() {
   for (int nx = 1; nx <= 512; ++nx)
     if (grad_h(nx) < 1 || (grad_w(nx) + 6) * (grad_h(nx) + 6) > kGradTile) return false;
@@ -2131,24 +2132,16 @@ __host__ __device__ constexpr size_t hybrid_smem_bytes(bool ns) {
          (NUC3D_HYB_PREFETCH ? rhs_stage_bytes<DIR>(ns) : 0);
 }
 
-// Cells of a launch.
-template <int DIR> inline long long launch_cells(const Launch &L) {
-  const BlockDev *h = L.h_blocks;
-  if (L.k1 > 0) return (long long)h[0].n[0] * h[0].n[1] * (L.k1 - L.k0);
-  long long n = 0;
-  for (int b = L.b0; b < (L.b1 > 0 ? L.b1 : L.tm_dir[DIR].nblocks); ++b) n += h[b].N;
-  return n;
-}
-
 // Which launches run pipelined (pipe_sweep_kernel) where they may.  It has half the warps per SM
 // of the one-tile-per-CTA sweep, but TMA brings its tiles, so it wins
 //   * where a scheme has little arithmetic: upwind1st everywhere (right-hand side, us, pipelined /
 //     tiles: reference-order Euler 64^3 108 / 130, 128^3 471 / 676, Navier-Stokes 128^3 1052 /
 //     1231; throughput Euler 64^3 80 / 90, 128^3 277 / 421, Navier-Stokes 128^3 727 / 869);
-//     weno3js of the throughput build (Euler 128^3 361 / 464, Navier-Stokes 765 / 911), along xi
-//     only with the eigenvalues, whose metrics the tiles wait for (without: 64^3 18.6 / 16.6,
-//     128^3 99 / 107); and weno3js of the reference-order build in launches of at most a tile per
-//     resident CTA (32^3 Euler 72 / 80, Navier-Stokes 96 / 109);
+//     weno3js of the throughput build along eta and zeta (Euler 128^3 386 / 464, Navier-Stokes
+//     784 / 911), and along xi with the eigenvalues, whose metrics the tiles wait for, from
+//     eight tiles per resident CTA on (128^3 361 / 386, 8 blocks of 40x36x44 149 / 158, 96^3
+//     220 / 229, a blast 258 / 253; 64^3 96 / 95); and weno3js of the reference-order build in
+//     launches of at most a tile per resident CTA (32^3 Euler 72 / 80, Navier-Stokes 96 / 109);
 //   * where a launch has a tile for every other SM at most: its time is then one tile's latency.
 //     Steps of 16^3, one context alone and three overlapping, per step: reference-order weno5js
 //     Navier-Stokes 211 / 225 and 76 / 80, WENO5-Z Euler 167 / 177 and 60 / 63; throughput eta
@@ -2159,20 +2152,17 @@ template <int DIR> inline long long launch_cells(const Launch &L) {
 // With more tiles and more arithmetic it is the slower one (reference-order WENO5-Z 64^3 xi 66 /
 // 55, eta 63 / 54, zeta 60 / 53, 128^3 440 / 364, 414 / 353, 390 / 358; throughput WENO7 128^3 xi
 // 268 / 212, eta 249 / 213).  Close to even: the throughput build's zeta, pipelined (WENO7 64^3
-// Navier-Stokes 45 / 41, 128^3 303 / 318, 8 blocks of 40x36x44 80 / 92), and the reference-order
-// weno3js of Euler, pipelined along zeta and, with the eigenvalues, xi where the tiles are at
-// least half full (right-hand side 128^3 813 / 848, 8 blocks of 40x36x44 312 / 330; tiles a
-// quarter full, 27 blocks of 16^3: 179 / 166; Navier-Stokes 64^3 250 / 242).
+// Navier-Stokes 45 / 41, 128^3 303 / 318, 8 blocks of 40x36x44 80 / 92), and weno3js in larger
+// launches of the reference-order build, tiles: pipelined along zeta and xi, smooth periodic
+// blocks gain and blasts with outlets lose (right-hand side, Euler: 128^3 813 / 848, 27 blocks of
+// 16^3 179 / 166; blast 128x128x96 689 / 629, 64^3 164 / 147).
 template <int DIR, int SCH>
 constexpr bool kPipe = !NUC3D_FAST || DIR != 0 || SCH == SCH_UPWIND1 || SCH == SCH_WENO3JS;
 template <int DIR, int SCH> inline bool pipe_pays(const Launch &L, int ntiles, int flags) {
-  const bool ns = (flags & SW_NS) != 0, eig = (flags & SW_EIG) != 0;
   if (SCH == SCH_UPWIND1 || (NUC3D_FAST && DIR == 2)) return true;
-  if (NUC3D_FAST && SCH == SCH_WENO3JS) return DIR == 1 || eig;
-  if (4 * ntiles <= L.pipe_grid) return DIR == 1 || (!NUC3D_FAST && (ns || SCH != SCH_WENO7JS));
-  if (NUC3D_FAST || SCH != SCH_WENO3JS) return false;
-  if (ntiles <= L.pipe_grid) return true;
-  return !ns && (DIR == 2 || (DIR == 0 && eig)) && 2 * launch_cells<DIR>(L) >= 256ll * ntiles;
+  if (NUC3D_FAST && SCH == SCH_WENO3JS) return DIR == 1 || ((flags & SW_EIG) && ntiles >= 8 * L.pipe_grid);
+  if (SCH == SCH_WENO3JS) return ntiles <= L.pipe_grid;
+  return 4 * ntiles <= L.pipe_grid && (DIR == 1 || (flags & SW_NS) || SCH != SCH_WENO7JS);
 }
 template <int DIR, int SCH> inline bool may_pipe(const Launch &L) {
   return kPipe<DIR, SCH> && L.d_maps && L.pipe_grid > 0 && ((L.pipe_dirs >> DIR) & 1) &&
@@ -2215,7 +2205,7 @@ inline cudaError_t launch_sweep_s(const Launch &L, int stage, int flags) {
 
 #if NUC3D_FAST
 template <int DIR> inline bool runs_marching(const Launch &L) {
-  return march_dir(L.P, DIR) && (DIR == 2 ? L.march_zeta : launch_cells<DIR>(L) >= kMarchMin);
+  return march_dir(L.P, DIR) && (DIR == 2 ? L.march_zeta : march_cells<DIR>(L) >= kMarchMin);
 }
 #endif
 

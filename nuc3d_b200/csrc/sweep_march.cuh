@@ -420,6 +420,15 @@ inline int march_length(const BlockDev *h, int b0, int b1, int dir, const MarchP
   return len;
 }
 
+// Cells of a launch.
+template <int DIR> inline long long march_cells(const Launch &L) {
+  const BlockDev *h = L.h_blocks;
+  if (L.k1 > 0) return (long long)h[0].n[0] * h[0].n[1] * (L.k1 - L.k0);
+  long long n = 0;
+  for (int b = L.b0; b < (L.b1 > 0 ? L.b1 : L.tm_dir[DIR].nblocks); ++b) n += h[b].N;
+  return n;
+}
+
 template <int DIR, int SCH, bool NSV, int RIE>
 inline cudaError_t launch_march_r(const Launch &L, int stage, int flags) {
   using M = MarchGeo<DIR, SCH, NSV>;
