@@ -184,9 +184,9 @@ compact_march_kernel(const BlockDev *__restrict__ blocks, TileMap tm, SolverPara
     }
     // (the faces outside the system, f < R and f > L - R, and its last row have no next face: times
     // a zero, a NaN or Inf of that face would reach them)
-    const bool in = f >= R && f < L - R;
-    xp = in ? a[1] - a[0] * xp : a[1];
-    xm = in ? a[3] - a[2] * xm : a[3];
+    if (f < R || f >= L - R) xp = xm = 0.0;
+    xp = a[1] - a[0] * xp;
+    xm = a[3] - a[2] * xm;
     const double h = xp + xm;
     if (f < L && live) {
       const long long idx = cell0 + f * sL;
