@@ -936,6 +936,11 @@ static bool slab_pipeline_ok(const nuc3d_ctx *c) {
   return c->blocks[0].n[2] >= 2 * tile_l(kHostZetaShape);
 }
 
+// The kernel of direction d's sweep over the whole context.
+static int sweep_kind(const nuc3d_ctx *c, int d) {
+  return c->exact ? nuc3d::exact::sweep_kind(c->L, d) : nuc3d::fast::sweep_kind(c->L, d);
+}
+
 #ifndef NUC3D_HOST_PIECES
 #define NUC3D_HOST_PIECES 8  // copy pieces per slab (256^3: 17.45 ms per step against 17.66 with 4)
 #endif
@@ -1176,16 +1181,27 @@ int nuc3d_solve_host(nuc3d_ctx *c, double *const *q_host, int nsteps) {
     CUDA_TRY(cudaStreamWaitEvent(c->stream, c->ev_h2d, 0));
     if (by_block) {
       // stages 0 and 1 whole; stage 2's ghost fluxes (and NS gradients) of every block,
-      // then each block's sweeps, whose last (zeta) releases that block's download
+      // then the sweeps of one block after the other, whose last (zeta) releases the block's
+      // download.  Where zeta marches, a launch takes blocks up to 2^16 cells: a smaller march
+      // lasts as long as one line's walk (80 blocks of 16^3 one by one: 4.15 ms a call), and the
+      // residual's partial sums are the march's, so tiles are no choice.
       CUDA_TRY(cudaMemsetAsync(&c->d_state->max_eig_bits, 0, sizeof(unsigned long long), c->stream));
       CUDA_TRY(c->stage(0, true, true));
       CUDA_TRY(c->stage(1, true, false));
       CUDA_TRY(run([&] { return nuc3d::fast::run_stage_pre(L, 2); },
                    [&] { return nuc3d::exact::run_stage_pre(L, 2); }));
-      for (int b = 0; b < nb; ++b) {
-        CUDA_TRY(run([&] { return nuc3d::fast::run_stage_sweeps(L, 2, b, b + 1); },
-                     [&] { return nuc3d::exact::run_stage_sweeps(L, 2, b, b + 1); }));
-        CUDA_TRY(cudaEventRecord(c->ev_zeta[b], c->stream));
+      long long left = 0;
+      for (int b = 0; b < nb; ++b) left += c->blocks[b].N;
+      const long long least = sweep_kind(c, 2) == SWEEP_MARCH ? 1 << 16 : 1;
+      for (int b0 = 0, b1 = 0; b0 < nb; b0 = b1) {
+        long long cells = 0;
+        while (b1 < nb && (cells < least || left < least)) {
+          cells += c->blocks[b1].N;
+          left -= c->blocks[b1++].N;
+        }
+        CUDA_TRY(run([&] { return nuc3d::fast::run_stage_sweeps(L, 2, b0, b1); },
+                     [&] { return nuc3d::exact::run_stage_sweeps(L, 2, b0, b1); }));
+        for (int b = b0; b < b1; ++b) CUDA_TRY(cudaEventRecord(c->ev_zeta[b], c->stream));
       }
       if (L.d_res_last)
         CUDA_TRY(run([&] { return nuc3d::fast::run_residual(L, false); },
@@ -1225,11 +1241,6 @@ static int apply_shapes(nuc3d_ctx *c, const int shape[3]) {
           c->L.tm_dir[d].tile_start[bi] + nuc3d::exact::tile_count(d, c->blocks[bi].n, shape[d]);
   c->drop_graph();
   return build_maps(c);
-}
-
-// The kernel of direction d's sweep over the whole context.
-static int sweep_kind(const nuc3d_ctx *c, int d) {
-  return c->exact ? nuc3d::exact::sweep_kind(c->L, d) : nuc3d::fast::sweep_kind(c->L, d);
 }
 
 static bool compact_scheme(int s) { return s == SCH_CRWENO5 || s == SCH_HCCS || s == SCH_HCCS77; }
