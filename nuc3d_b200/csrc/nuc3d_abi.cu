@@ -1306,24 +1306,33 @@ int nuc3d_autotune(nuc3d_ctx *c, int reps, int shape_out[3], double ms_out[9]) {
     CUDA_TRY(cudaEventCreate(&ev.b));
     cudaEvent_t e0 = ev.a, e1 = ev.b;
     int cur[3] = {c->L.shape[0], c->L.shape[1], c->L.shape[2]};
-    // every tile shape of every explicit direction, each pipelined and one tile per CTA
-    // where the pipelined sweeps apply (the pipeline's bit for a direction is its choice)
+    // every tile shape of every explicit direction, and where its launch would run pipelined,
+    // also one tile per CTA (the pipeline's bit for a direction is its choice; where no launch
+    // is pipelined it stays).  A direction that marches has one kernel, whatever its shape and
+    // bit: it is timed as it stands, and both stay for the smaller launches that take tiles
     const int mask0 = c->pipe_mask;
-    const bool can_pipe = c->L.d_maps != nullptr;
     int mask = mask0;
     for (int d = 0; d < 3; ++d) {
       if (compact_scheme(c->P.scheme[d])) { best[d] = 0; continue; }
       double tbest = 1e300;
-      int best_mode = (mask0 >> d) & 1;
+      const int mode0 = (mask0 >> d) & 1;
+      int best_mode = mode0;
+      const bool march = sweep_kind(c, d) == SWEEP_MARCH;
+      const int sh0 = march ? cur[d] : 0, sh1 = march ? cur[d] + 1 : kTileShapes;
       // two passes over the candidates, each keeping its faster time: one disturbed
       // measurement cannot decide the choice
       for (int pass = 0; pass < 2; ++pass)
-      for (int sh = 0; sh < kTileShapes; ++sh) {
-        for (int mode = can_pipe ? 1 : 0; mode >= 0; --mode) {
+      for (int sh = sh0; sh < sh1; ++sh) {
+        bool choice = false;  // the two modes are two kernels
+        for (int mode = 1; mode >= 0; --mode) {
           cur[d] = sh;
           mask = (mask & ~(1 << d)) | (mode << d);
           c->pipe_mask = mask;
           if (int r = apply_shapes(c, cur)) return r;
+          if (mode == 1) {
+            choice = sweep_kind(c, d) == SWEEP_PIPE;
+            if (!choice) continue;
+          }
           auto sweep = [&]() {
             return c->exact ? nuc3d::exact::run_sweep(c->L, d, 0, 0) : nuc3d::fast::run_sweep(c->L, d, 0, 0);
           };
@@ -1340,7 +1349,11 @@ int nuc3d_autotune(nuc3d_ctx *c, int reps, int shape_out[3], double ms_out[9]) {
             return fail(NUC3D_ECUDA, "autotune: a pipelined sweep timed out");
           const double ms = (double)t / reps;
           if (ms_out && (ms_out[3 * d + sh] < 0.0 || ms < ms_out[3 * d + sh])) ms_out[3 * d + sh] = ms;
-          if (ms < tbest || (ms == tbest && sh < best[d])) { tbest = ms; best[d] = sh; best_mode = mode; }
+          if (ms < tbest || (ms == tbest && sh < best[d])) {
+            tbest = ms;
+            best[d] = sh;
+            best_mode = choice ? mode : mode0;
+          }
         }
       }
       cur[d] = best[d];
