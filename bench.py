@@ -328,7 +328,7 @@ def ours(args):
             s.set_pipeline(args.pipe_mask if args.pipe_mask > 1 else bool(args.pipe_mask))
     else:
         tiles = s.autotune(reps=3)["shape"]
-    pipe_dirs_step = s.pipeline()  # directions the timed steps run pipelined (bit d)
+    pipe_dirs_step = s.pipeline()  # directions whose sweeps may run pipelined (bit d)
 
     def barrier():
         if dist is not None:
